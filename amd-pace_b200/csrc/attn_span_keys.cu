@@ -363,7 +363,8 @@ int sm_count() {
 }
 
 template <int N>
-int launch_keys(KeysParams& p, const CUtensorMap& tk, const CUtensorMap& tpage, int max_tokens, int max_keys, int entries, cudaStream_t s) {
+int launch_keys(KeysParams& p, const CUtensorMap& tk, const CUtensorMap& tpage, int64_t q_rows, int max_tokens, int max_keys, int entries,
+                cudaStream_t s) {
   const int smem = keys_smem(N, p.k_blocks, p.dv16).total;
   if (smem > 227 * 1024 - 64) return PACE_ERR_UNSUPPORTED;
   p.tmem_cols = 128;
@@ -378,8 +379,8 @@ int launch_keys(KeysParams& p, const CUtensorMap& tk, const CUtensorMap& tpage, 
   int ns = 1;
   for (int k = 2; k <= 8 && units * k <= sm_count(); ++k)
     if ((pages + k - 1) / k < (pages + ns - 1) / ns) ns = k;
-  CUtensorMap tq;
-  const uint64_t dims[2] = {(uint64_t)p.q_elems, (uint64_t)p.st.n_tokens * p.H}, str[1] = {(uint64_t)p.q_elems * 2};
+  CUtensorMap tq;   // (the box of a last tile goes on behind its rows: what the buffer does not hold must lie outside the map)
+  const uint64_t dims[2] = {(uint64_t)p.q_elems, (uint64_t)q_rows * p.H}, str[1] = {(uint64_t)p.q_elems * 2};
   const uint32_t box[2] = {64, N};
   const int rc = tensor_map_bf16(&tq, p.q, 2, dims, str, box);
   if (rc != PACE_OK) return rc;
@@ -439,8 +440,9 @@ int attn_span_keys(const pace_kv_pool_t* pl, int layer, const pace_step_t& st, c
   if (rc == PACE_OK) rc = tensor_map_bf16(&tpage, p.kv.k, 3, dims, str, whole);
   if (rc != PACE_OK) return rc;
   const int E = a.entry_end - a.entry_begin;
-  return a.max_tokens * p.Gq <= 16 ? launch_keys<16>(p, tk, tpage, a.max_tokens, a.max_keys, E, s)
-                                   : launch_keys<32>(p, tk, tpage, a.max_tokens, a.max_keys, E, s);
+  const int64_t q_rows = a.q_rows ? a.q_rows : st.n_tokens;
+  return a.max_tokens * p.Gq <= 16 ? launch_keys<16>(p, tk, tpage, q_rows, a.max_tokens, a.max_keys, E, s)
+                                   : launch_keys<32>(p, tk, tpage, q_rows, a.max_tokens, a.max_keys, E, s);
 }
 
 }  // namespace pace

@@ -103,7 +103,7 @@ inline bool span_args_ok(const pace_step_t* st, const pace_attn_span_args_t* a, 
   return a && a->q && a->out && a->n_q_heads >= 1 && n_kv_heads >= 1 && a->n_q_heads % n_kv_heads == 0 && a->dim >= 1 &&
          a->vdim >= 1 && a->q_elems >= a->dim && a->out_elems >= a->vdim && a->entry_begin >= 0 &&
          a->entry_end >= a->entry_begin && a->entry_end <= st->n_entries && a->max_tokens >= 0 && a->max_keys >= 0 && a->softcap >= 0.f &&
-         (a->out_row == 0 || a->out_row >= (int64_t)a->n_q_heads * a->out_elems) &&
+         a->q_rows >= 0 && (a->out_row == 0 || a->out_row >= (int64_t)a->n_q_heads * a->out_elems) &&
          (a->dtype == PACE_DTYPE_BF16 || a->dtype == PACE_DTYPE_FP32) && a->span >= PACE_SPAN_ALL &&
          a->span <= PACE_SPAN_CHUNK && (a->span == PACE_SPAN_ALL || a->span_size >= 1);
 }

@@ -96,7 +96,7 @@ class AttnSpanArgs(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("q", "out", "slopes", "sinks")] + \
                [(n, C.c_int32) for n in ("n_q_heads", "dim", "vdim", "dtype", "q_elems", "out_elems", "entry_begin", "entry_end",
                                          "max_tokens", "max_keys", "span", "span_size")] + \
-               [("scale", C.c_float), ("softcap", C.c_float), ("out_row", C.c_int64)]
+               [("scale", C.c_float), ("softcap", C.c_float), ("out_row", C.c_int64), ("q_rows", C.c_int64)]
 
 
 class AttnSpanPrefillArgs(C.Structure):

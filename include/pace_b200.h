@@ -534,7 +534,7 @@ int pace_attn_general(const pace_kv_pool_t* pool, int32_t layer, const pace_step
  * NULL: no bias), and exp(sinks[h]) is added to the denominator (sinks NULL: ordinary softmax).  Query head h reads KV head h / (n_q_heads / n_kv_heads).
  * Row t of q (dtype [n_tokens][n_q_heads][q_elems], dim elements used, zero up to the next multiple of 8) and of out
  * ([n_tokens][n_q_heads][out_elems], vdim elements written; tokens out_row elements apart where that is not 0) belongs to
- * token t.  The pool holds the step's own rows already;
+ * token t; q may end behind the last token of the entries (q_rows).  The pool holds the step's own rows already;
  * lengths come from the step.  PACE_ROWS_SHARED pools: the value is the first vdim elements of the key row.
  * Scores, weights and sums are fp32 (with bf16 rows the weights enter the second product as two bf16 terms).
  * max_tokens / max_keys: upper bounds, over the entries, of their tokens and of their last position + 1.
@@ -554,6 +554,7 @@ typedef struct {
   float scale;
   float softcap;         /* 0: none */
   int64_t out_row;       /* elements between the tokens of out; 0: n_q_heads * out_elems */
+  int64_t q_rows;        /* tokens that q holds, from the step's first one on (nothing behind them is read); 0: n_tokens */
 } pace_attn_span_args_t;
 int pace_attn_span(const pace_kv_pool_t* pool, int32_t layer, const pace_step_t* step, const pace_attn_span_args_t* a,
                    void* stream);
