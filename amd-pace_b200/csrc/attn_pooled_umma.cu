@@ -15,13 +15,14 @@
 #include <algorithm>
 
 #include "pooled.cuh"
+#include "pooled_sums.h"
 #include "umma.cuh"
 
 namespace pace {
 namespace {
 
 constexpr int kChunk = 64, kBlockBytes = kChunk * 128, kMaxStages = 6, kKeyStages = 3;
-constexpr int kGroups = 4, kCols = kChunk / kGroups, kSoftmax = 128 * kGroups, kThreads = kSoftmax + 96;   // softmax: warpgroups, their columns
+constexpr int kGroups = PooledSums::kGroups, kCols = kChunk / kGroups, kSoftmax = 128 * kGroups, kThreads = kSoftmax + 96;   // softmax: warpgroups, their columns
 constexpr int kSlots = 4;
 constexpr uint32_t kColO = kSlots * kChunk, kColsO = 512 - kColO;
 constexpr float kLazy = 8.0f;  // log2 units a row's maximum may grow before O is rescaled
@@ -218,14 +219,14 @@ __device__ __forceinline__ void pooled_softmax(const PooledParams& p, Bars& b, u
       const float inv = l > 0.f ? 1.0f / l : 0.f;
       const bool opens = gk == un.g0, closes = gk + 1 == un.g1;
       // a lane mixes four columns of one token for up to four of its heads: item = (token, part of its heads, four columns)
-      const int per = rounds * 4 * kUmmaRows;          // a piece's sums
-      float4* acc = p.acc + (size_t)u * p.nv * pieces * per + row;
+      const PooledSums sums = {un.nv, pieces, rounds};
+      float4* acc = p.acc + (size_t)u * PooledSums{p.nv, pieces, rounds}.size() + row;
       float4 y[4];                                     // the sums so far of the next item
-      auto ask = [&](int at, bool live_piece) {
+      auto ask = [&](int at) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) y[k] = opens || !live_piece ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldcg(acc + at + k * kUmmaRows);
+        for (int k = 0; k < 4; ++k) y[k] = opens || at < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldcg(acc + at + k * kUmmaRows);
       };
-      ask(grp * per, true);
+      ask(sums.first(grp));
       if (!gave_up) gave_up = !umma_issuer_wait(pv, pv_phase, abort);
       tc_fence_after();
       float* mine = sm.o[grp][row];
@@ -240,15 +241,12 @@ __device__ __forceinline__ void pooled_softmax(const PooledParams& p, Bars& b, u
             *reinterpret_cast<float4*>(mine + q * 4) = make_float4(__uint_as_float(raw[4 * q]) * inv, __uint_as_float(raw[4 * q + 1]) * inv,
                                                                    __uint_as_float(raw[4 * q + 2]) * inv, __uint_as_float(raw[4 * q + 3]) * inv);
           __syncwarp();
-          const int at = (j * pieces + d) * per;
           for (int r = 0; r < rounds; ++r) {
             const int it = r * 32 + lane;
             const int h4 = r == 0 ? item_h4 : (it >> 2) % parts4 * 4, tl = r == 0 ? item_tok : (it >> 2) / parts4;
             const bool there = it < items;
             float4 z[4] = {y[0], y[1], y[2], y[3]};
-            if (r + 1 < rounds) ask(at + (r + 1) * 4 * kUmmaRows, true);
-            else if (d + kGroups < pieces) ask(at + kGroups * per, true);
-            else ask(((j + 1) * pieces + grp) * per, j + 1 < un.nv);
+            ask(sums.next(grp, j, d, r));
             const float* o = sm.o[grp][(row & ~31) + (there ? tl * p.Gq : 0)] + (lane & 3) * 4;
             const float* f = mix_j + (there ? h4 : 0);
             const int tk = un.tok0 + warp * p.tpw + tl, col = d * 16 + (lane & 3) * 4;
@@ -271,7 +269,7 @@ __device__ __forceinline__ void pooled_softmax(const PooledParams& p, Bars& b, u
             }
             if (!closes) {
 #pragma unroll
-              for (int k = 0; k < 4; ++k) __stcg(acc + at + (r * 4 + k) * kUmmaRows, z[k]);
+              for (int k = 0; k < 4; ++k) __stcg(acc + sums.at(j, d, r) + k * kUmmaRows, z[k]);
             } else if (store) {
 #pragma unroll
               for (int k = 0; k < 4; ++k) {
@@ -539,8 +537,8 @@ Plan plan_units(int n_entries, int max_tokens, int H, int G, int vdim, bool mixe
   p.n_sub = (G + most - 1) / most;
   p.nv = (G + p.n_sub - 1) / p.n_sub;
   p.n_sub = (G + p.nv - 1) / p.nv;
-  p.bytes = mixed && G > 1 ? (uint64_t)n_entries * p.n_tiles * p.n_sub * p.nv * ((vdim + 15) / 16) *
-                                      ((p.tpw * ((H / G + 3) / 4) * 4 + 31) / 32) * 16 * kUmmaRows * sizeof(float) : 0;
+  const PooledSums sums = {p.nv, (vdim + 15) / 16, (p.tpw * ((H / G + 3) / 4) * 4 + 31) / 32};
+  p.bytes = mixed && G > 1 ? (uint64_t)n_entries * p.n_tiles * p.n_sub * sums.size() * sizeof(float4) : 0;
   return p;
 }
 bool plan_ok(int H, int G, int vdim) { return H >= 1 && G >= 1 && H % G == 0 && H / G <= 32 && vdim >= 1 && vdim <= 128; }
