@@ -12,7 +12,7 @@ Differences that come from the path being on the GPU:
   * RoPE is fused into the append kernel (``update_cache_rope``); a residual sum and the norm behind it are one
     kernel, the activation of the MLP another; projections are library products, one for weights that lie side
     by side (query, key and value; gate and up).  Where gradients, hooks or replaced modules are in play the
-    layers run as separate torch ops;
+    modules are called one by one;
   * ``forward_tokens`` takes only the NEW tokens and allows ragged counts per sequence, which
     batched speculative decoding needs; ``forward`` is the reference signature on top of it.
 """
@@ -23,6 +23,8 @@ import numpy as np
 import torch
 import torch.nn.functional as F
 from torch import nn
+from torch.autograd import forward_ad
+from torch.nn.modules.module import _has_any_global_hook
 
 from pace_b200 import _C
 from pace_b200.llm.cache import KVCacheBase, KVCacheManager
@@ -32,21 +34,24 @@ from pace_b200.ops import MultiHeadAttention, RotaryEmbedding
 from pace_b200.ops.linear import linear
 
 
-def _lin(module: nn.Linear, x: torch.Tensor) -> torch.Tensor:
-    """``module(x)``; a decode step's few token rows take the weight-streaming kernel (ops/linear.py)."""
-    return linear(x, module.weight, module.bias)
+def _untouched(m: nn.Module, cls: type) -> bool:
+    """Whether calling m is nothing but ``cls.forward``: no other class, no forward of its own, no hooks."""
+    return type(m) is cls and "forward" not in m.__dict__ and not (
+        m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or _has_any_global_hook())
 
 
 def _no_graph(*tensors: torch.Tensor) -> bool:
-    """Whether kernels that autograd does not see may run over these tensors."""
+    """Whether kernels that autograd, transforms and tracers do not see may run over these tensors."""
+    if forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active() or torch.jit.is_tracing() or torch.compiler.is_compiling():
+        return False
     grad = torch.is_grad_enabled()
-    return all(t.is_cuda and t.dtype == torch.bfloat16 and t.numel() > 0 and not (grad and t.requires_grad) for t in tensors)
+    return all(type(t) in (torch.Tensor, nn.Parameter) and t.is_cuda and t.dtype == torch.bfloat16 and t.numel() > 0 and
+               not (grad and t.requires_grad) for t in tensors)
 
 
 def _fusable(x: torch.Tensor, *modules: nn.Module) -> bool:
     """The same for plain linears over x that nobody has replaced or hooked."""
-    return all(type(m) is nn.Linear and m.bias is None and not m._forward_hooks and not m._forward_pre_hooks for m in modules) and \
-        _no_graph(x, *(m.weight for m in modules))
+    return all(_untouched(m, nn.Linear) and m.bias is None for m in modules) and _no_graph(x, *(m.weight for m in modules))
 
 
 def _side_by_side(*modules: nn.Module) -> Optional[torch.Tensor]:
@@ -75,12 +80,18 @@ def _lay_out(*modules: nn.Module) -> None:
         at += x.shape[0]
 
 
+def _rows(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """x as the append reads it: that type, heads of consecutive elements, rows at 16 bytes (what a replaced projection leaves may differ)."""
+    if x.dtype != dtype or x.stride(-1) != 1 or any(s % 8 for s in x.stride()[:-1]) or x.data_ptr() % 16:
+        x = x.to(dtype).clone(memory_format=torch.contiguous_format)
+    return x
+
+
 def _add_norm(x: torch.Tensor, y: Optional[torch.Tensor], norm: "RMSNorm"):
     """(x + y, its norm); without y (x, its norm)."""
     W = x.shape[-1]
-    if type(norm) is RMSNorm and _no_graph(x, norm.weight, x if y is None else y) and W % 8 == 0 and W <= 8192 and \
+    if _untouched(norm, RMSNorm) and _no_graph(x, norm.weight, x if y is None else y) and W % 8 == 0 and W <= 8192 and \
             norm.weight.is_contiguous() and x.is_contiguous() and (y is None or (y.is_contiguous() and y.shape == x.shape)) and \
-            not norm._forward_hooks and not norm._forward_pre_hooks and \
             not any(t.data_ptr() % 16 for t in ((x, norm.weight) if y is None else (x, y, norm.weight))):
         s, out = x if y is None else torch.empty_like(x), torch.empty_like(x)
         torch.ops.pace_b200.add_norm(x, y, norm.weight, None if y is None else s, out, norm.eps)
@@ -124,8 +135,8 @@ class LlamaMLP(nn.Module):
                 both = linear(x, w).view(-1, 2 * n)
                 act = torch.empty(both.shape[0], n, dtype=x.dtype, device=x.device)
                 torch.ops.pace_b200.glu(both, act, _C.ACT_SILU)
-                return _lin(self.down_proj, act.view(*x.shape[:-1], n))
-        return _lin(self.down_proj, _lin(self.up_proj.linear, x) * F.silu(_lin(self.gate_proj.linear, x)))
+                return self.down_proj(act.view(*x.shape[:-1], n))
+        return self.down_proj(up(x) * F.silu(gate(x)))
 
 
 class FusedRope:
@@ -153,10 +164,10 @@ class LlamaAttention(nn.Module):
         self.attention = MultiHeadAttention()
 
     def project(self, hidden: torch.Tensor):
-        """Query, key and value heads ``[..., heads, D]``; one product where the weights lie side by side."""
+        """Query, key and value heads ``[..., heads, D]``; one product where the weights lie side by side, otherwise the modules' own."""
         parts = (self.q_proj, self.k_proj, self.v_proj)
         w = _side_by_side(*parts) if _fusable(hidden, *parts) else None
-        x = linear(hidden, w).split([m.weight.shape[0] for m in parts], -1) if w is not None else [_lin(m, hidden) for m in parts]
+        x = linear(hidden, w).split([m.weight.shape[0] for m in parts], -1) if w is not None else [m(hidden) for m in parts]
         return [t.unflatten(-1, (-1, self.head_dim)) for t in x]
 
     def forward(self, hidden_states, position_embeddings, kv_cache: KVCacheBase, kv_start=None, n_new=None,
@@ -172,11 +183,11 @@ class LlamaAttention(nn.Module):
             key_h, value_h = kv_cache.update_cache(k, v.transpose(1, 2), concat_dim=2, n_new_per_seq=n_new)
         out = self.attention(q, key_h, value_h, attention_mask=None, kv_start=kv_start, q_lens=q_lens)
         out = out.transpose(1, 2).reshape(bsz, q_len, -1)
-        return _lin(self.o_proj, out)
+        return self.o_proj(out)
 
     def forward_packed(self, hidden: torch.Tensor, pk: "Packed", kv_cache: KVCacheBase) -> torch.Tensor:
         """``hidden`` [T, hidden]: the step's tokens of all sequences, back to back."""
-        q, k, v = self.project(hidden)
+        q, k, v = (_rows(t, pk.q.dtype) for t in self.project(hidden))
         q, key_h, value_h = kv_cache.update_cache_rope_packed(q, k, v, pk.row_at, pk.counts, pk.q_lens, pk.rope.table_row, pk.rope.op, pk.q)
         out = self.attention(q, key_h, value_h, attention_mask=None, q_lens=pk.q_lens)
         return self.o_proj(out.transpose(1, 2).reshape(-1, self.num_heads * self.head_dim).index_select(0, pk.staged))
@@ -201,8 +212,8 @@ class Packed:
         self.live = [b for b, c in enumerate(self.counts) if c]
         parts = [np.asarray(list(cached), dtype=np.int64), cu[1:][n > 0] - 1, np.asarray(self.live, dtype=np.int64),
                  bidx * n_max + np.arange(T) - cu[:-1][bidx], np.concatenate([n, cu[:-1]]).astype(np.int32).view(np.int64)]
-        if tokens is not None and not tokens.is_cuda:
-            parts.append(tokens.reshape(-1).numpy().astype(np.int64))
+        if tokens is not None and tokens.device.type == "cpu" and tokens.dim() == 1 and tokens.dtype in (torch.int32, torch.int64):
+            parts.append(tokens.numpy().astype(np.int64))
         host = torch.from_numpy(np.concatenate(parts))
         dev = host.pin_memory().to(device, non_blocking=True) if torch.device(device).type == "cuda" else host.to(device)
         views = dev.split([len(p) for p in parts])
@@ -238,7 +249,7 @@ class LlamaDecoderLayer(nn.Module):
 
     @property
     def plain(self) -> bool:
-        return type(self) is LlamaDecoderLayer and not self._forward_hooks and not self._forward_pre_hooks
+        return _untouched(self, LlamaDecoderLayer)
 
 
 class LlamaModel(nn.Module):
@@ -276,7 +287,7 @@ class LlamaModel(nn.Module):
         hidden = self.embed_tokens(tokens)
         y = None
         for idx, layer in enumerate(self.layers):
-            if type(layer) is LlamaDecoderLayer:
+            if type(layer) is LlamaDecoderLayer and "forward_packed" not in layer.__dict__:
                 hidden, y = layer.parts(hidden, y, lambda n: layer.self_attn.forward_packed(n, pk, kv_cache[idx]))
             else:
                 hidden, y = layer.forward_packed(hidden if y is None else hidden + y, pk, kv_cache[idx]), None
@@ -309,7 +320,7 @@ class LlamaForCausalLM(nn.Module):
         if bool((mask == 0).any()):
             kv_start = (mask.cumsum(-1) == 0).sum(-1).to(torch.int32)
         hidden = self.model.forward_tokens(new_ids, kv_cache, position_ids, kv_start)
-        return ModelOutput(logits=_lin(self.lm_head, hidden))
+        return ModelOutput(logits=self.lm_head(hidden))
 
     # -- ragged form used by batched speculative decoding ---------------------------------------
     def forward_ragged(self, new_ids: torch.Tensor, n_new: Sequence[int], kv_cache: KVCacheManager) -> ModelOutput:
@@ -321,7 +332,7 @@ class LlamaForCausalLM(nn.Module):
         position_ids.clamp_(max=self.config.max_position_embeddings - 1)
         ragged = None if all(n == new_ids.shape[1] for n in n_new) else list(n_new)
         hidden = self.model.forward_tokens(new_ids, kv_cache, position_ids, None, ragged)
-        return ModelOutput(logits=_lin(self.lm_head, hidden))
+        return ModelOutput(logits=self.lm_head(hidden))
 
 
     def forward_device_ragged(self, new_ids: torch.Tensor, n_new: torch.Tensor, kv_cache: KVCacheManager,
@@ -335,7 +346,7 @@ class LlamaForCausalLM(nn.Module):
         position_ids = base + torch.arange(new_ids.shape[1], device=new_ids.device).unsqueeze(0)
         position_ids.clamp_(max=self.config.max_position_embeddings - 1)
         hidden = self.model.forward_tokens(new_ids, kv_cache, position_ids, None, n_new)
-        return ModelOutput(logits=_lin(self.lm_head, hidden))
+        return ModelOutput(logits=self.lm_head(hidden))
 
     # -- packed form used by continuous batching ----------------------------------------------------
     def forward_packed(self, tokens: torch.Tensor, counts: Sequence[int], kv_cache: KVCacheManager,
@@ -366,10 +377,11 @@ class LlamaForCausalLM(nn.Module):
     def _lay_out(self) -> None:
         """Weights that a step multiplies the same rows by lie side by side: query, key and value; gate and up."""
         for layer in self.model.layers:
-            if type(layer) is LlamaDecoderLayer:
-                at, mlp = layer.self_attn, layer.mlp
-                _lay_out(at.q_proj, at.k_proj, at.v_proj)
-                _lay_out(mlp.gate_proj.linear, mlp.up_proj.linear)
+            if type(layer) is LlamaDecoderLayer and type(layer.self_attn) is LlamaAttention:
+                _lay_out(layer.self_attn.q_proj, layer.self_attn.k_proj, layer.self_attn.v_proj)
+            if type(layer) is LlamaDecoderLayer and type(layer.mlp) is LlamaMLP and \
+                    type(layer.mlp.gate_proj) is type(layer.mlp.up_proj) is _FusedLinear:
+                _lay_out(layer.mlp.gate_proj.linear, layer.mlp.up_proj.linear)
 
     def load_weights(self, tensors: Dict[str, torch.Tensor]) -> None:
         """Checkpoint names: the reference's state dict, or the plain ``mlp.up_proj.weight`` form of it."""

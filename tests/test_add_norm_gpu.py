@@ -81,4 +81,92 @@ def test_weights_side_by_side_give_the_same_layer():
     hook = at.k_proj.register_forward_hook(lambda *a: seen.append(1))
     with torch.no_grad():
         assert all(torch.equal(a, b) or (a.float() - b.float()).norm() <= 0.01 * b.float().norm() for a, b in zip(at.project(x), proj))
+    assert seen == [1]
     hook.remove()
+
+
+class Doubled(torch.nn.Module):
+    """A projection with a forward of its own over a plain linear, as adapters are; fp32 out, rows that lie apart."""
+
+    def __init__(self, base):
+        super().__init__()
+        self.base, self.weight, self.bias = base, base.weight, None
+
+    def forward(self, x):
+        return torch.cat([self.base(x).float() * 2, self.base(x[..., :1].expand_as(x)).float()], -1)[..., : self.weight.shape[0]]
+
+
+def tiny_llama(layers=2):
+    from pace_b200.llm.models.llama import LlamaForCausalLM
+    cfg = SimpleNamespace(hidden_size=256, intermediate_size=512, num_hidden_layers=layers, num_attention_heads=4, num_key_value_heads=2,
+                          vocab_size=64, max_position_embeddings=128, rope_theta=1e4, rms_norm_eps=1e-5, rope_scaling=None)
+    torch.manual_seed(1)
+    return LlamaForCausalLM(cfg).to(DEV, torch.bfloat16), cfg
+
+
+def packed_logits(model, cfg, counts=(7, 3)):
+    from pace_b200.llm.cache import KVCacheManager, KVCacheType
+    mgr = KVCacheManager(cfg, 32, KVCacheType.BMC)
+    ids = torch.arange(sum(counts)) % cfg.vocab_size
+    return model.forward_packed(ids, list(counts), mgr, rows=range(len(ids))).logits
+
+
+def close(a, b):
+    return (a.double() - b.double()).norm() <= 0.03 * b.double().norm()
+
+
+def test_packed_pass_calls_replaced_and_hooked_modules():
+    model, cfg = tiny_llama()
+    with torch.no_grad():
+        want = packed_logits(model, cfg)
+        for name in ("q_proj", "k_proj", "v_proj", "o_proj"):
+            seen = []
+            hooks = [getattr(lay.self_attn, name).register_forward_hook(lambda m, a, y: seen.append(1) or y) for lay in model.model.layers]
+            assert close(packed_logits(model, cfg), want) and seen == [1, 1], name
+            for h in hooks:
+                h.remove()
+        for name in ("q_proj", "v_proj"):
+            at = model.model.layers[0].self_attn
+            base = getattr(at, name)
+            setattr(at, name, Doubled(base))
+            got = packed_logits(model, cfg)
+            setattr(at, name, base)
+            base.weight.data.mul_(2)
+            assert close(got, packed_logits(model, cfg)) and not close(got, want), name
+            base.weight.data.mul_(0.5)
+        model.model.layers[1].self_attn.q_proj.bias = torch.nn.Parameter(torch.ones(256, dtype=torch.bfloat16, device=DEV))
+        assert not close(packed_logits(model, cfg), want)
+        model.model.layers[1].self_attn.q_proj.bias = None
+        assert torch.equal(packed_logits(model, cfg), want)
+
+
+def test_forwards_of_single_objects_are_called():
+    """A forward put on one layer, norm or projection, as offloading wrappers do."""
+    from pace_b200.llm.cache import KVCacheManager, KVCacheType
+    model, cfg = tiny_llama()
+    ids = torch.arange(12, device=DEV).view(2, 6)
+
+    def logits():
+        return model(ids, kv_cache=KVCacheManager(cfg, 32, KVCacheType.BMC), attention_mask=torch.ones_like(ids)).logits
+    with torch.no_grad():
+        want = logits()
+        lay = model.model.layers[0]
+        for m in (lay, lay.input_layernorm, model.model.norm, lay.self_attn.v_proj, lay.mlp.gate_proj.linear):
+            seen, own = [], m.forward
+            m.forward = lambda *a, **k: seen.append(1) or own(*a, **k)          # noqa: B023
+            got = logits()
+            del m.forward
+            assert seen and close(got, want), type(m)
+            with torch.nn.modules.module.register_module_forward_hook(lambda mod, a, y: seen.append(2) if mod is m else None):
+                assert close(logits(), want) and 2 in seen, type(m)
+
+
+def test_transforms_see_the_whole_mlp():
+    model, _ = tiny_llama(1)
+    mlp = model.model.layers[0].mlp.requires_grad_(False)
+    x, dx = torch.randn(4, 256, device=DEV).bfloat16(), torch.randn(4, 256, device=DEV).bfloat16()
+    up, gate, down = (m.weight.double() for m in (mlp.up_proj.linear, mlp.gate_proj.linear, mlp.down_proj))
+    _, want = torch.func.jvp(lambda t: (t @ up.T * torch.nn.functional.silu(t @ gate.T)) @ down.T, (x.double(),), (dx.double(),))
+    _, got = torch.func.jvp(mlp, (x,), (dx,))
+    assert close(got, want)
+    assert close(torch.func.vmap(mlp)(x), mlp(x))
