@@ -710,8 +710,7 @@ __global__ void __launch_bounds__(threads_of(UMMA, UMMA ? 8 : MT * NS), (!UMMA &
     if (b < p.batch) {
       my_slot[r] = view_slot(p.kv, b);
       if (my_slot[r] >= 0) {
-        // (ahead of the wait from L2: lines of an earlier kernel may still lie in L1)
-        my_len[r] = (early_general && p.kv.seq_len ? __ldcg(p.kv.seq_len + my_slot[r]) : view_len(p.kv, my_slot[r])) + (pend ? 1 : 0);
+        my_len[r] = view_len(p.kv, my_slot[r]) + (pend ? 1 : 0);
         // the producer will walk this row of the block table a few microseconds from now: start
         // bringing its first lines into L2 (the K/V stream of the previous launch has evicted them)
         if (p.kv.block_table) {

@@ -116,9 +116,12 @@ __device__ __forceinline__ void raise_status(int32_t* status, int bits) {
   if (status) atomicOr(status, bits);
 }
 
+// Slots, lengths and block-table entries are read from L2: an attention launch looks them up ahead of its wait, beside the kernel in
+// front of it, on SMs whose L1 may still hold what a line was before an older kernel wrote it.
+
 // slot of batch row b, or -1 when out of range (status raised)
 __device__ __forceinline__ int view_slot(const KVView& kv, int b) {
-  int s = kv.seq_ids ? kv.seq_ids[b] : b + kv.slot_base;
+  int s = kv.seq_ids ? __ldcg(kv.seq_ids + b) : b + kv.slot_base;
   if (s < 0 || s >= kv.max_seqs) {
     raise_status(kv.status, PACE_DEV_BAD_INDEX);
     return -1;
@@ -126,7 +129,7 @@ __device__ __forceinline__ int view_slot(const KVView& kv, int b) {
   return s;
 }
 __device__ __forceinline__ int view_len(const KVView& kv, int slot) {
-  return kv.seq_len ? kv.seq_len[slot] : kv.fixed_len;
+  return kv.seq_len ? __ldcg(kv.seq_len + slot) : kv.fixed_len;
 }
 // physical page of logical page lp of a slot, or -1
 __device__ __forceinline__ int view_page(const KVView& kv, int slot, int lp) {
@@ -152,7 +155,7 @@ struct PageWindow {
   __device__ __forceinline__ int load(int l) const {
     if (!row) return slot;
     if (l < 0 || l >= max_pages) return -1;
-    const int pg = __ldg(row + l);
+    const int pg = __ldcg(row + l);
     return (pg < 0 || pg >= n_pages) ? -1 : pg;
   }
   // step: how far the window moves at a time (a multiple of the pages one chunk spans, <= 32)
