@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_states_kernel(pace_step_t s
   unsigned char *hi = smem, *mid = smem + 2 * kBlock, *vt = smem + 4 * kBlock;
   Sync& sy = *reinterpret_cast<Sync*>(smem + 4 * kBlock + VP / 64 * kBlock);
   Item it;
-  if (!find_item(st, blockIdx.z, &it)) return;
+  if (!find_item(st, a.place0 + blockIdx.z, &it)) return;
   const int h = blockIdx.y, vb = blockIdx.x, v0 = vb * VP, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const __nv_bfloat16* rows = a.src + (size_t)it.t0 * a.src_stride;
   Rows<128> k;
@@ -252,20 +252,23 @@ __global__ void __launch_bounds__(kThreads) chunk_prefix_kernel(pace_step_t st, 
   const int e = blockIdx.z, h = blockIdx.y / a.v_blocks, vb = blockIdx.y % a.v_blocks;
   const int u = blockIdx.x * kThreads + threadIdx.x, p = (u >> 3) % (VP / 8), row = (u / VP) * 8 + (u & 7), col = vb * VP + p * 8;
   const int cu = st.cu[e], count = st.cu[e + 1] - cu, n = (count + kChunk - 1) / kChunk;
-  const bool fresh = st.start[e] == 0, mine = row < a.dim && col < a.vdim;
+  // this round's chunks [c_a, c_z) of the sequence; the state comes in with its first chunk and between rounds
+  const int at = cu / kChunk + e - a.place0, c_a = max(0, -at), c_z = min(n, a.places - at);
+  if (c_a >= c_z) return;
+  const bool fresh = st.start[e] == 0 && c_a == 0, mine = row < a.dim && col < a.vdim;
   float* state = a.state + (((size_t)st.slot[e] * a.heads + h) * a.dim + row) * a.vdim + col;
   float s[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) s[j] = 0.f;
   if (!fresh && mine) Vec<float, 8>::load(state, s);
-  const size_t step = (size_t)a.heads * a.v_blocks, first = (size_t)(cu / kChunk + e) * step + blockIdx.y;
+  const int64_t step = (int64_t)a.heads * a.v_blocks, first = at * step + blockIdx.y;
   const float full = SSD ? 0.f : powf(a.decay[h], (float)kChunk), rest = SSD ? 0.f : powf(a.decay[h], (float)(count - (n - 1) * kChunk));
   constexpr int kBatch = 4;                                // chunks whose loads are in flight together
-  for (int c0 = 0; c0 < n; c0 += kBatch) {
+  for (int c0 = c_a; c0 < c_z; c0 += kBatch) {
     float x[kBatch][8], f[kBatch];
 #pragma unroll
     for (int b = 0; b < kBatch; ++b)
-      if (c0 + b < n) {
+      if (c0 + b < c_z) {
         const size_t place = first + (c0 + b) * step;
         Vec<float, 8>::load(a.add + place * (kChunk * VP) + add_at<VP>(row, p), x[b]);
         if constexpr (SSD) f[b] = a.log_decay[place];
@@ -273,7 +276,7 @@ __global__ void __launch_bounds__(kThreads) chunk_prefix_kernel(pace_step_t st, 
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) {
       const int c = c0 + b;
-      if (c >= n) break;
+      if (c >= c_z) break;
       if (c > 0 || !fresh) {
         unsigned char* to = a.tiles + (first + c * step) * (4 * kChunk * VP) + tile_at(row, p);
         uint32_t hi[4], lo[4];
@@ -302,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_out_kernel(pace_step_t st, 
   unsigned char *sh = kt, *sl = VP == 64 ? kt + kV : vt;
   Sync& sy = *reinterpret_cast<Sync*>(smem + 4 * kBlock + kV);
   Item it;
-  if (!find_item(st, blockIdx.z, &it)) return;
+  if (!find_item(st, a.place0 + blockIdx.z, &it)) return;
   const int h = blockIdx.y, vb = blockIdx.x, v0 = vb * VP, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const size_t place = ((size_t)blockIdx.z * a.heads + h) * a.v_blocks + vb;
   const bool state = it.c > 0 || st.start[it.e] != 0;      // (a sequence that begins here begins from zeros)
@@ -473,8 +476,7 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_out_kernel(pace_step_t st, 
 }
 
 template <bool SSD, int VP>
-int launch(const pace_step_t& st, const ChunkArgs& a, cudaStream_t s) {
-  const dim3 grid((unsigned)a.v_blocks, (unsigned)a.heads, (unsigned)a.places);
+int launch(const pace_step_t& st, ChunkArgs a, int places, cudaStream_t s) {
   constexpr int kV = VP / 64 * kBlock, smem = 4 * kBlock + kV + (int)sizeof(Sync);
   static bool configured[16] = {};
   int dev = 0;
@@ -484,30 +486,39 @@ int launch(const pace_step_t& st, const ChunkArgs& a, cudaStream_t s) {
     PACE_CUDA_TRY(cudaFuncSetAttribute(chunk_out_kernel<SSD, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     if (dev < 16) configured[dev] = true;
   }
-  chunk_states_kernel<SSD, VP><<<grid, kThreads, smem, s>>>(st, a);
-  PACE_LAUNCH_CHECK("chunk_states_kernel");
-  chunk_prefix_kernel<SSD, VP><<<dim3(kChunk * VP / 8 / kThreads, (unsigned)(a.heads * a.v_blocks), (unsigned)st.n_entries), kThreads, 0, s>>>(st, a);
-  PACE_LAUNCH_CHECK("chunk_prefix_kernel");
-  chunk_out_kernel<SSD, VP><<<grid, kThreads, smem, s>>>(st, a);
-  PACE_LAUNCH_CHECK("chunk_out_kernel");
+  for (const int per = a.places; a.place0 < places; a.place0 += per) {
+    a.places = places - a.place0 < per ? places - a.place0 : per;
+    const dim3 grid((unsigned)a.v_blocks, (unsigned)a.heads, (unsigned)a.places);
+    chunk_states_kernel<SSD, VP><<<grid, kThreads, smem, s>>>(st, a);
+    PACE_LAUNCH_CHECK("chunk_states_kernel");
+    chunk_prefix_kernel<SSD, VP><<<dim3(kChunk * VP / 8 / kThreads, (unsigned)(a.heads * a.v_blocks), (unsigned)st.n_entries), kThreads, 0, s>>>(st, a);
+    PACE_LAUNCH_CHECK("chunk_prefix_kernel");
+    chunk_out_kernel<SSD, VP><<<grid, kThreads, smem, s>>>(st, a);
+    PACE_LAUNCH_CHECK("chunk_out_kernel");
+  }
   return PACE_OK;
 }
 
-struct Parts { uint64_t add, tiles, kv, log_decay, total; int places, v_blocks; };
+// Scratch of a round of launches; all places of a step together, or as many as the budget holds: a step of many tokens goes through in
+// rounds, the states of the sequences that a round leaves in the middle wait where they belong.  4096 tokens of 32 lightning heads take
+// 198 MB and one round; 16384 of 64 heads 1.5 GB at once 988 us, in rounds of 512 MB 1074, 256 MB 1157, 128 MB 1274, 32 MB 2157.
+constexpr uint64_t kBudget = 512ull << 20;
+struct Parts { uint64_t add, tiles, kv, log_decay, total; int places, per_round, v_blocks; };
 Parts parts_of(const pace_step_t& st, int heads, int vdim, bool lightning) {
   Parts p;
   const int vp = vdim <= 64 ? 64 : 128;
   p.places = st.n_tokens / kChunk + st.n_entries;
   p.v_blocks = (vdim + vp - 1) / vp;
-  const uint64_t n = (uint64_t)p.places * heads * p.v_blocks;
-  p.add = n * kChunk * vp * 4;
-  p.tiles = n * kChunk * vp * 4;
-  p.kv = lightning ? n * (2 * kBlock + (uint64_t)kChunk * vp * 2) : 0;
+  const uint64_t items = (uint64_t)heads * p.v_blocks, add = (uint64_t)kChunk * vp * 4, kv = lightning ? 2 * kBlock + (uint64_t)kChunk * vp * 2 : 0;
+  const uint64_t fit = kBudget / (items * (2 * add + kv + 4));
+  p.per_round = fit < 1 ? 1 : fit < (uint64_t)p.places ? (int)fit : p.places;
+  const uint64_t n = (uint64_t)p.per_round * items;
+  p.add = p.tiles = n * add;
+  p.kv = n * kv;
   p.log_decay = lightning ? 0 : (n * 4 + 255) / 256 * 256;
   p.total = p.add + p.tiles + p.kv + p.log_decay;
   return p;
 }
-constexpr uint64_t kMostScratch = 2ull << 30;
 // Prompts that are a chunk at most stay with the chunks of 64, which take one launch: 128 tokens 24.1 us (lightning) and 20.8 (state space)
 // against 24.7 and 26.8 here; 200 tokens 42.0 and 31.6 against 24.9 and 26.9.
 constexpr int kFewTokens = kChunk + 1;
@@ -517,8 +528,8 @@ constexpr int kFewTokens = kChunk + 1;
 uint64_t chunk_umma_bytes(const pace_step_t& st, int heads, int dim, int vdim, bool lightning) {
   if (dim <= 64 || dim > 128 || dim % 8 || vdim % 8 || heads > 65535 || st.n_entries > 65535 || st.max_count < kFewTokens) return 0;
   const Parts p = parts_of(st, heads, vdim, lightning);
-  if (p.places > 65535 || (int64_t)heads * p.v_blocks > 65535) return 0;
-  return p.total <= kMostScratch ? p.total : 0;
+  if (p.per_round > 65535 || (int64_t)heads * p.v_blocks > 65535) return 0;
+  return p.total <= kBudget + 256 ? p.total : 0;
 }
 
 bool chunk_umma_fits(const pace_step_t& st, const ChunkArgs& a, const void* workspace, uint64_t workspace_bytes) {
@@ -531,13 +542,13 @@ int chunk_umma(const pace_step_t& st, ChunkArgs a, void* workspace, cudaStream_t
   const bool lightning = a.decay != nullptr;
   const Parts p = parts_of(st, a.heads, a.vdim, lightning);
   unsigned char* w = static_cast<unsigned char*>(workspace);
-  a.places = p.places, a.v_blocks = p.v_blocks;
+  a.place0 = 0, a.places = p.per_round, a.v_blocks = p.v_blocks;
   a.add = reinterpret_cast<float*>(w);
   a.tiles = w + p.add;
   a.kv = a.tiles + p.tiles;
   a.log_decay = reinterpret_cast<float*>(a.kv + p.kv);
-  if (lightning) return a.vdim <= 64 ? launch<false, 64>(st, a, s) : launch<false, 128>(st, a, s);
-  return a.vdim <= 64 ? launch<true, 64>(st, a, s) : launch<true, 128>(st, a, s);
+  if (lightning) return a.vdim <= 64 ? launch<false, 64>(st, a, p.places, s) : launch<false, 128>(st, a, p.places, s);
+  return a.vdim <= 64 ? launch<true, 64>(st, a, p.places, s) : launch<true, 128>(st, a, p.places, s);
 }
 
 }  // namespace pace

@@ -18,8 +18,8 @@ struct ChunkArgs {
   __nv_bfloat16* out;
   int64_t out_stride;
   int heads, dim, vdim;
-  // scratch (chunk_umma_bytes)
-  int places, v_blocks;
+  // scratch (chunk_umma_bytes) and the places of one round of launches
+  int place0, places, v_blocks;
   float *add, *log_decay;
   unsigned char *tiles, *kv;
 };

@@ -70,3 +70,61 @@ def test_ssd(lens, H, G, D, P):
     torch.ops.pace_b200.ssd_prefill(step.handle, x, dt_raw, bias, neg_a, skip, S, out, G)
     _close(out, want, 2.0 ** -8)
     _close(S, state, 2e-5)        # exponentials of sums of up to 128 log decays: some ulp of 32 bits each
+
+
+def _lightning_case(lens, H, D, P, seed=3):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    x = torch.randn(sum(lens), H * (2 * D + P), device=DEV, generator=g).bfloat16()
+    starts = [9 if b % 2 else 0 for b in range(len(lens))]
+    S = torch.randn(len(lens), H, D, P, device=DEV, generator=g)
+    return x, torch.full((H,), 0.99, device=DEV), S, starts
+
+
+@pytest.mark.parametrize("lens", [[4000, 1, 129, 3000], [130] * 60 + [700, 5000]])
+def test_rounds_of_launches(lens):
+    """Steps whose scratch is more than one round of launches may hold: the same as every sequence by itself."""
+    from pace_b200 import _C
+    from pace_b200.ops import hybrid
+    H, D, P = 64, 128, 128
+    x, decay, S, starts = _lightning_case(lens, H, D, P)
+    step = _step(lens, starts)
+    places = sum(lens) // 128 + len(lens)
+    got_bytes = _C.lib.pace_lightning_scratch_bytes(step.struct, H, D, P, _C.DTYPE_BF16)
+    assert got_bytes < places * H * 192 * 1024          # more than one round
+    states = S.clone()
+    got, at = hybrid.lightning(step, x, decay, states), 0
+    for row in step.rows:
+        n, one = lens[row], S[row: row + 1].clone()
+        want = hybrid.lightning(_step([n], [starts[row]]), x[at: at + n], decay, one)
+        # a chunk's products and sums are the same in either; sequences that fit the older chunks alone differ in rounding
+        tol = 0 if n > 128 else 2.0 ** -8
+        assert (got[at: at + n].double() - want.double()).norm() <= tol * want.double().norm()
+        assert (states[row].double() - one[0].double()).norm() <= (0 if n > 128 else 1e-4) * one.double().norm()
+        at += n
+
+
+@pytest.mark.parametrize("room", [0, 40])
+def test_less_room_takes_the_smaller_chunks(room):
+    """Where the scratch of the chunks of 128 cannot be had, those of 64 run in theirs."""
+    from pace_b200 import _C
+    from pace_b200.ops import hybrid
+    lens, H, D, P = [4096], 16, 128, 128
+    x, decay, S, starts = _lightning_case(lens, H, D, P)
+    step = _step(lens, starts)
+    a, b = S.clone(), S.clone()
+    want = hybrid.lightning(step, x, decay, a)
+    out = torch.empty_like(want)
+    need = _C.lib.pace_lightning_scratch_bytes(step.struct, H, D, P, _C.DTYPE_BF16)
+    fewer = _C.lib.pace_lightning_workspace_bytes(1, 4096, H, D, P)
+    assert fewer < 40 << 20 < need
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.set_per_process_memory_fraction(min(1.0, (torch.cuda.memory_reserved() + ((room or 1 << 14) << 20)) /
+                                                   torch.cuda.get_device_properties(0).total_memory))
+    try:
+        torch.ops.pace_b200.lightning_prefill(step.handle, x, decay, b, out)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(out, want) == (room == 0)         # (the other chunks ran)
+    _close(out, want.double(), 2.0 ** -8)
+    _close(b, a.double(), 1e-4)
