@@ -7,6 +7,8 @@
 // four rows each.  Keys and values pass through shared memory 32 at a time: a lane scores one key for its
 // warp's rows, then owns value columns while the weights are passed round by shuffles.  Online softmax,
 // everything in fp32.
+#include <type_traits>
+
 #include "span.cuh"
 
 namespace pace {
@@ -170,8 +172,8 @@ int launch_general(const KVView& kv, const pace_step_t& st, const GeneralArgs& a
 // ---- 32-bit rows ---------------------------------------------------------------------------------------------------------------
 // The kernel above issues a shared-memory load per 4 multiply-adds of a lane and a shuffle per 4 of the second product: 3.3 TFLOP/s of
 // the 74 that the FMA units have (two prompts of 701 and 1100 tokens, 16/4 heads of 128: 2102 us).  Register tiles instead: a block of four warps owns 64 rows, a
-// thread 8 of them with 4 of a tile's 64 keys, then with 4 or 8 value columns, so that a 16-byte shared-memory load feeds 11 to 21
-// multiply-adds.  The rows' operands are the same for 16 lanes (one shared-memory pass), keys and values pass by cp.async while the other
+// thread 8 of them with 4 of a tile's 64 keys, then with 4 or 8 value columns, so that a 16-byte shared-memory load feeds 11 (scores,
+// values of up to 64 elements) to 16 multiply-adds.  The rows' operands are the same for 16 lanes (one shared-memory pass), keys and values pass by cp.async while the other
 // product runs, and two blocks fit an SM, so that one's barriers and exponentials run beside the other's products.  The same prompts:
 // 240 us with the append, 30 TFLOP/s, bound by FMA issue and, in blocks of few keys, by the latency of a tile's chain.  fp32 throughout; a
 // score is the sum of two chains (even and odd elements, the halves of a two-wide FMA), which makes neither sum longer: against 64 bits
@@ -244,6 +246,11 @@ __global__ void __launch_bounds__(kTileThreads, 2) attn_tile_kernel(KVView kv, p
   const int n_keys = last_hi + 1, first_hi = span_first(a.span, a.span_size, last_hi);
   const int k_begin = span_first(a.span, a.span_size, last_lo) / kTileKeys * kTileKeys;
   const bool full = r0 + kTileRows <= rows;
+  // ... and the rows of the warp: values that a row does not see (later tokens, tokens in front of a span) stay out of its sums, where a
+  // weight of zero would still hand on an infinity or NaN
+  const int wr = r0 + 16 * (threadIdx.x >> 5);
+  const int w_lo = wr < rows ? start + wr / Gq : -1, w_hi = wr < rows ? start + (min(wr + 16, rows) - 1) / Gq : -1;
+  const int w_first = span_first(a.span, a.span_size, max(w_lo, 0)), w_all = span_first(a.span, a.span_size, max(w_hi, 0));
   const float* kp = static_cast<const float*>(static_cast<const void*>(kv.k));
   const float* vp = static_cast<const float*>(static_cast<const void*>(kv.v));
 
@@ -364,27 +371,35 @@ __global__ void __launch_bounds__(kTileThreads, 2) attn_tile_kernel(KVView kv, p
       __syncwarp();                                     // a warp reads the weights it wrote itself
       const float* pr = ps + my_row * S::kPLd;
       const float* vr = vs + kh * 32 * DP + 4 * cl;
+      const int p0 = k0 + 32 * kh, j_a = max(0, w_first - p0), j_z = min(32, w_hi + 1 - p0);   // (the same for the warp)
+      auto add_values = [&](auto ragged) {
+        constexpr bool some = decltype(ragged)::value;
 #pragma unroll 2
-      for (int j = 0; j < kTileKeys / 2; j += 4) {
-        float4 pp[8];
+        for (int j = some ? j_a & ~3 : 0; j < (some ? j_z : 32); j += 4) {
+          float4 pp[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) pp[i] = *reinterpret_cast<const float4*>(pr + 2 * i * S::kPLd + j);
+          for (int i = 0; i < 8; ++i) pp[i] = *reinterpret_cast<const float4*>(pr + 2 * i * S::kPLd + j);
 #pragma unroll
-        for (int y = 0; y < 4; ++y) {
-          float4 v[kHalves];
+          for (int y = 0; y < 4; ++y) {
+            if (some && (j + y < j_a || j + y >= j_z)) continue;
+            float4 v[kHalves];
 #pragma unroll
-          for (int h = 0; h < kHalves; ++h) v[h] = *reinterpret_cast<const float4*>(vr + (j + y) * DP + 64 * h);
+            for (int h = 0; h < kHalves; ++h) v[h] = *reinterpret_cast<const float4*>(vr + (j + y) * DP + 64 * h);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float w = y == 0 ? pp[i].x : y == 1 ? pp[i].y : y == 2 ? pp[i].z : pp[i].w;
+            for (int i = 0; i < 8; ++i) {
+              const float w = y == 0 ? pp[i].x : y == 1 ? pp[i].y : y == 2 ? pp[i].z : pp[i].w;
+              if (some && w == 0.f) continue;
 #pragma unroll
-            for (int h = 0; h < kHalves; ++h) {
-              fma2(acc[i][2 * h], make_float2(w, w), make_float2(v[h].x, v[h].y));
-              fma2(acc[i][2 * h + 1], make_float2(w, w), make_float2(v[h].z, v[h].w));
+              for (int h = 0; h < kHalves; ++h) {
+                fma2(acc[i][2 * h], make_float2(w, w), make_float2(v[h].x, v[h].y));
+                fma2(acc[i][2 * h + 1], make_float2(w, w), make_float2(v[h].z, v[h].w));
+              }
             }
           }
         }
-      }
+      };
+      if (p0 >= w_all && p0 + 31 <= w_lo) add_values(std::false_type{});   // (every row sees all of them)
+      else add_values(std::true_type{});
     }
     __syncthreads();
     if (more) fetch(vp, vd, vs, DP, off + (buf ^ 1) * kTileKeys);

@@ -407,9 +407,10 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_out_kernel(pace_step_t st, 
     const uint32_t v_lo = desc_lo(vt, kBlock);
     constexpr uint32_t IDESC = umma_idesc(VP, true);
     if (ok && leader) {
+      // (rows in front of a step's 16 tokens stay out of it: zero weights would hand on an infinity or NaN among later values)
       for (int t = 0; t < 2; ++t)
         for (int s = 0; s < steps; ++s)
-          umma_bf16_ts(tO, tS + t * 64 + s * 8, pack64(v_lo + s * (2048 >> 4), kDescHi), IDESC, t | s ? 1u : 0u);
+          umma_bf16_ts(tO, tS + t * 64 + s * 8, pack64(v_lo + s * (2048 >> 4), kDescHi), IDESC, t | s ? 1u : 0u, s * 16);
       umma_commit(&sy.values);
     }
     __syncwarp();

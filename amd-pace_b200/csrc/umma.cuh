@@ -85,15 +85,16 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a_desc, uint
       : "r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
-// A operand in tensor memory (128 lanes x 8 columns of packed bf16 pairs per 16-wide k-step)
+// A operand in tensor memory (128 lanes x 8 columns of packed bf16 pairs per 16-wide k-step); the first `off` rows are left as they are
 __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
+                                             uint32_t accumulate, int off = 0) {
+  auto mask = [&](int w) -> uint32_t { return off >= 32 * w + 32 ? 0xffffffffu : off > 32 * w ? (1u << (off - 32 * w)) - 1u : 0u; };
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
       :
-      : "r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(mask(0)), "r"(mask(1)), "r"(mask(2)), "r"(mask(3))
       : "memory");
 }
 // Blackwell's two-wide fp32 arithmetic and three-input maximum: a row of 64 scores takes 32 instructions

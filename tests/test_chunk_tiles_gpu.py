@@ -128,3 +128,28 @@ def test_less_room_takes_the_smaller_chunks(room):
     assert torch.equal(out, want) == (room == 0)         # (the other chunks ran)
     _close(out, want.double(), 2.0 ** -8)
     _close(b, a.double(), 1e-4)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("bad", [0, 15, 16, 77, 127, 128, 200])
+def test_values_of_later_tokens_stay_out(bad, value):
+    """A token's infinity or NaN among its values reaches no token in front of its 16."""
+    from pace_b200.ops import hybrid
+    n, H, D, P, G = 260, 2, 128, 72, 1
+    g = torch.Generator(device=DEV).manual_seed(bad)
+    step, keep = _step([n], [0]), bad // 16 * 16
+    x = torch.randn(n, H * (2 * D + P), device=DEV, generator=g).bfloat16()
+    decay = torch.full((H,), 0.9, device=DEV)
+    y = x.clone()
+    y[bad, 2 * H * D:] = value
+    want, got = (hybrid.lightning(step, t, decay, torch.zeros(1, H, D, P, device=DEV)) for t in (x, y))
+    assert torch.equal(got[:keep], want[:keep]) and not torch.isfinite(got[bad]).all()
+    x = torch.randn(n, H * P + 2 * G * D, device=DEV, generator=g).bfloat16()
+    y = x.clone()
+    y[bad, : H * P] = value
+    dt, bias, neg_a, skip = torch.randn(n, H, device=DEV, generator=g).bfloat16(), *(torch.rand(3, H, device=DEV, generator=g) - 1)
+    outs = []
+    for t in (x, y):
+        outs.append(torch.empty(n, H * P, device=DEV, dtype=torch.bfloat16))
+        torch.ops.pace_b200.ssd_prefill(step.handle, t, dt, bias, neg_a, skip, torch.zeros(1, H, D, P, device=DEV), outs[-1], G)
+    assert torch.equal(outs[1][:keep], outs[0][:keep]) and not torch.isfinite(outs[1][bad]).all()
