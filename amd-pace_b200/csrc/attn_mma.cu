@@ -24,6 +24,7 @@
 #include <climits>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "umma.cuh"
@@ -207,6 +208,71 @@ static_assert(sizeof(ResMeta) == 64, "ResMeta is one 64-byte line");
 namespace pace {
 namespace {
 
+// The merge of a cut unit's partials by its last arriver, into the output rows.  A thread has four columns of a row at a time, AT partials'
+// loads in flight together (a round trip per group of them), IT such places side by side.  own: this CTA's part, read from shared memory
+// (-1: none).  Mostly one warp does this, and a unit of 20 rows of 128 is 20 round trips for it: with two columns and eight partials at a
+// time (40, and for two to four partials twice the arithmetic) verify passes of 12 x 5 tokens behind 300, eight layers, took 415 us, with
+// two columns and four partials 346, so 216; 16 x 4 behind 200 to 2000, 4 KV heads 355, 240, 212; decode of one sequence of 3000 232, -, 211.
+template <int D, int MR, int NTHR, int AT, int IT>
+__device__ __forceinline__ void merge_parts(const float* recs, int first_slot, int parts, int own, const float* rnum, const float* rM,
+                                            const float* rden, int t, int live, int r_lo, int G, __nv_bfloat16* out, int64_t o_sh, int64_t o_ss) {
+  constexpr int REC = MR * (D + 2);
+  for (int o0 = t * 4; o0 < live * D; o0 += NTHR * 4 * IT) {
+    float M[IT], den[IT], num[IT][4];
+#pragma unroll
+    for (int i = 0; i < IT; ++i) M[i] = -INFINITY, den[i] = num[i][0] = num[i][1] = num[i][2] = num[i][3] = 0.f;
+    for (int c0 = 0; c0 < parts; c0 += AT) {
+      float mc[IT][AT], dc[IT][AT], nn[IT][AT][4];
+#pragma unroll
+      for (int i = 0; i < IT; ++i) {
+        const int oi = o0 + i * NTHR * 4, row = oi / D;
+#pragma unroll
+        for (int k = 0; k < AT; ++k) {
+          const int c = c0 + k;
+          mc[i][k] = -INFINITY;
+          dc[i][k] = nn[i][k][0] = nn[i][k][1] = nn[i][k][2] = nn[i][k][3] = 0.f;
+          if (i > 0 && oi >= live * D) continue;
+          if (c == own) {
+            mc[i][k] = rM[row];
+            dc[i][k] = rden[row];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) nn[i][k][x] = rnum[oi + x];
+          } else if (c < parts) {
+            const float* r = recs + ((size_t)c * 2 + (c == 0 ? first_slot : 0)) * REC;
+            mc[i][k] = __ldcg(r + MR * D + row);
+            dc[i][k] = __ldcg(r + MR * D + MR + row);
+            *reinterpret_cast<float4*>(nn[i][k]) = __ldcg(reinterpret_cast<const float4*>(r + oi));
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < AT; ++k)
+#pragma unroll
+        for (int i = 0; i < IT; ++i) {
+          const float Mn = fmaxf(M[i], mc[i][k]);
+          if (Mn != -INFINITY) {
+            const float a = (M[i] == -INFINITY) ? 0.f : fast_exp2(M[i] - Mn);
+            const float f = (mc[i][k] == -INFINITY) ? 0.f : fast_exp2(mc[i][k] - Mn);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) num[i][x] = num[i][x] * a + nn[i][k][x] * f;
+            den[i] = den[i] * a + dc[i][k] * f;
+            M[i] = Mn;
+          }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      const int oi = o0 + i * NTHR * 4, row = oi / D, d = oi - row * D;
+      if (i > 0 && oi >= live * D) break;
+      const float inv = den[i] > 0.f ? 1.0f / den[i] : 0.f;
+      const int rr = r_lo + row, sq = rr / G, g = rr - sq * G;
+      uint32_t* to = reinterpret_cast<uint32_t*>(out + (size_t)g * o_sh + (size_t)sq * o_ss + d);
+      to[0] = f2_to_bf2(num[i][0] * inv, num[i][1] * inv);
+      to[1] = f2_to_bf2(num[i][2] * inv, num[i][3] * inv);
+    }
+  }
+}
+
 // Takes one finished unit part from its shared-memory result slot to global memory: the output
 // rows (mode 0), or an fp32 partial plus the arrival count and, for the last arriver, the merge
 // of all partials.  Run by a group of NTHR threads: one warp (WARP) or the eight consumer warps.
@@ -214,7 +280,6 @@ template <int D, int MR, int NTHR, bool WARP>
 __device__ __forceinline__ void publish_part(const MmaParams& p, const ResMeta& rm, const float* rnum, const float* rM,
                                              const float* rden, int t, int cta, int* flag) {
   constexpr int REC = MR * (D + 2);
-  constexpr int kAtOnce = 8;  // partials whose loads the merge has in flight: a round trip per group of them
   const int G = p.G, live = rm.live;
   auto group_sync = [&]() {
     if (WARP) __syncwarp(); else csync<NTHR>();
@@ -271,47 +336,16 @@ __device__ __forceinline__ void publish_part(const MmaParams& p, const ResMeta& 
   if (!is_last) return;
   __threadfence();
   }  // own < 0
-  for (int oi = t * 2; oi < live * D; oi += NTHR * 2) {
-    const int row = oi / D, d = oi - row * D;
-    float M = -INFINITY, n0 = 0.f, n1 = 0.f, den = 0.f;
-    for (int c0 = 0; c0 < rm.parts; c0 += kAtOnce) {  // (their loads in flight together)
-      float mc[kAtOnce], dc[kAtOnce];
-      float2 nn[kAtOnce];
-#pragma unroll
-      for (int k = 0; k < kAtOnce; ++k) {
-        const int c = c0 + k;
-        mc[k] = -INFINITY;
-        dc[k] = 0.f;
-        nn[k] = make_float2(0.f, 0.f);
-        if (c == own) {
-          mc[k] = rM[row];
-          dc[k] = rden[row];
-          nn[k] = *reinterpret_cast<const float2*>(rnum + oi);
-        } else if (c < rm.parts) {
-          const float* r = p.parts + ((size_t)(rm.first_cta + c) * 2 + (c == 0 ? rm.first_slot : 0)) * REC;
-          mc[k] = __ldcg(r + MR * D + row);
-          dc[k] = __ldcg(r + MR * D + MR + row);
-          nn[k] = __ldcg(reinterpret_cast<const float2*>(r + oi));
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < kAtOnce; ++k) {
-        const float Mn = fmaxf(M, mc[k]);
-        if (Mn != -INFINITY) {
-          const float a = (M == -INFINITY) ? 0.f : fast_exp2(M - Mn);
-          const float f = (mc[k] == -INFINITY) ? 0.f : fast_exp2(mc[k] - Mn);
-          n0 = n0 * a + nn[k].x * f;
-          n1 = n1 * a + nn[k].y * f;
-          den = den * a + dc[k] * f;
-          M = Mn;
-        }
-      }
-    }
-    const float inv = den > 0.f ? 1.0f / den : 0.f;
-    const int rr = rm.r_lo + row, sq = rr / G, g = rr - sq * G;
-    *reinterpret_cast<uint32_t*>(p.out + (size_t)rm.b * p.o_sb + (size_t)(rm.h * G + g) * p.o_sh + (size_t)sq * p.o_ss +
-                                 d) = f2_to_bf2(n0 * inv, n1 * inv);
-  }
+  const float* recs = p.parts + (size_t)rm.first_cta * 2 * REC;
+  __nv_bfloat16* out = p.out + (size_t)rm.b * p.o_sb + (size_t)rm.h * G * p.o_sh;
+  auto merge = [&](auto at_once, auto places) {
+    merge_parts<D, MR, NTHR, decltype(at_once)::value, decltype(places)::value>(recs, rm.first_slot, rm.parts, own, rnum, rM, rden, t, live,
+                                                                                rm.r_lo, G, out, p.o_sh, p.o_ss);
+  };
+  // (the eight consumer warps have few places each: two partials at a time leave their registers to the kernel's loops)
+  if (!WARP) merge(std::integral_constant<int, 2>{}, std::integral_constant<int, 1>{});
+  else if (rm.parts <= 2) merge(std::integral_constant<int, 2>{}, std::integral_constant<int, 2>{});
+  else merge(std::integral_constant<int, 4>{}, std::integral_constant<int, 1>{});
 }
 
 // One warp stores the pending K and V row of (sequence b, kv head h) in their slot of the pool: row
@@ -775,13 +809,7 @@ __global__ void __launch_bounds__(threads_of(UMMA, UMMA ? 8 : MT * NS), (!UMMA &
   }
   __syncthreads();
   T = prefix[n_items];
-  const long long T_real = misc[0];
-  const int share = max(kMinShare, (misc[2] + UC + kMaxParts - 1) / kMaxParts);
-  const long long most = MT == 1 || UMMA ? (T + share - 1) / share : T;
-  NC = T_real == 0 ? 1 : (long long)gridDim.x < most ? (int)gridDim.x : (int)most;
-  small = (T + 1) * (NC + 1) < (1LL << 31);
-  x0 = cta < NC ? range_begin(cta) : 0;
-  x1 = cta < NC ? range_begin(cta + 1) : 0;
+  const int T_real = misc[0];
   // When giving every CTA the same number of WHOLE units keeps the busiest CTA within 1.3x of an equal share of the
   // chunks, do that instead: a little more streaming for the busiest CTA (and some SMs idle), but no unit
   // is cut, so nothing is published to and merged from the workspace and no CTA waits for a last
@@ -792,15 +820,24 @@ __global__ void __launch_bounds__(threads_of(UMMA, UMMA ? 8 : MT * NS), (!UMMA &
   const int per_cta = (n_units + (int)gridDim.x - 1) / (int)gridDim.x;  // whole units per CTA
   // p.whole_units: the caller asked for this form whatever the balance; such a launch never touches
   // the workspace.
-  if (p.whole_units || (long long)per_cta * misc[2] * gridDim.x * 10 <= T_real * 13 + (MT == 1 ? (long long)gridDim.x * 10 * kWholeFree : 0)) {
-    x0 = x1 = 0;
+  if (p.whole_units || (long long)per_cta * misc[2] * gridDim.x * 10 <= (long long)T_real * 13 + (MT == 1 ? (long long)gridDim.x * 10 * kWholeFree : 0)) {
     const int u0 = cta * per_cta, u1 = min(n_units, u0 + per_cta);
+#pragma unroll 1
+    for (int u = u0; u < u1; ++u) n_my += chunks_in(u / Hkv);
     if (u0 < n_units) {
       const int it0 = u0 / Hkv, h0 = u0 - it0 * Hkv;
       x0 = (long long)prefix[it0] + (long long)h0 * ((prefix[it0 + 1] - prefix[it0]) / Hkv);
       const int it1 = (u1 - 1) / Hkv, h1 = (u1 - 1) - it1 * Hkv;
       x1 = (long long)prefix[it1] + (long long)(h1 + 1) * ((prefix[it1 + 1] - prefix[it1]) / Hkv);
     }
+  } else {
+    const int share = max(kMinShare, (misc[2] + UC + kMaxParts - 1) / kMaxParts);
+    const unsigned most = MT == 1 || UMMA ? ((unsigned)T + share - 1) / share : (unsigned)T;
+    NC = gridDim.x < most ? (int)gridDim.x : (int)most;
+    small = (T + 1) * (NC + 1) < (1LL << 31);
+    x0 = cta < NC ? range_begin(cta) : 0;
+    x1 = cta < NC ? range_begin(cta + 1) : 0;
+    if (x1 > x0) n_my = UC ? chunks_between(x0, x1) : (int)(x1 - x0);
   }
 
   if (warp != NW || any_empty || x1 <= x0) gdc_wait();
@@ -819,7 +856,6 @@ __global__ void __launch_bounds__(threads_of(UMMA, UMMA ? 8 : MT * NS), (!UMMA &
     }
   }
   if (x1 <= x0) return;
-  n_my = UC ? chunks_between(x0, x1) : (int)(x1 - x0);
   if (n_my <= 0) {
     gdc_wait();
     return;

@@ -30,7 +30,9 @@ def test_cut_units(lens, ctas):
         assert all(not got[i][b].any() for b in range(B) if not lens[b])
 
 
-@pytest.mark.parametrize("new,past", [([1, 300, 64, 2, 129, 0, 65], 0), ([1500, 3, 1], 70), ([9] * 5, 1000), ([12, 0, 9, 11], 3000), ([70] * 23, 1)])
+@pytest.mark.parametrize("new,past", [([1, 300, 64, 2, 129, 0, 65], 0), ([1500, 3, 1], 70), ([9] * 5, 1000), ([12, 0, 9, 11], 3000), ([70] * 23, 1),
+                                      # 12 to 32 rows of a unit: cut in two, in a few, in many parts (one warp merges them)
+                                      ([3], 3000), ([4, 0, 4, 3], 700), ([5] * 12, 300), ([8, 1, 7], 2000), ([6] * 40, 500), ([5], 9000)])
 def test_cut_units_of_many_query_rows(new, past):
     """Prompts and verify passes whose units are cut by position: tokens at the edges of tiles, sequences that sit out."""
     from pace_b200.llm.cache import KVCacheManager, KVCacheType
