@@ -53,7 +53,12 @@ constexpr int kMaxItems = 1024;
 //    the tile is drained.  Five prompts of 131 to 1709 tokens, 32 heads 215 (no cost) -> 120 (4), 117 (8), 121 (14); one of 1700
 //    tokens 133 -> 84, 82, 84; eight portions of 400 tokens behind up to 3600 218 -> 178, 161, 172; 9-token passes over 64 to 4000
 //    cached tokens 50 -> 36 or less.
-constexpr int kUnitCost = 4, kUnitCostWide = 8, kMinShare = 4, kMaxParts = 16, kWholeFree = 8;
+//  * Sixteen parts of a long unit are too few: the merge they save costs the same at any length, the stream they leave to few CTAs grows.
+//    A share ends at kMaxShare chunks (units of more than about 32000 tokens).  One, two and three sequences of 131072 tokens, bf16, heads
+//    of 128, us per launch - cut by the grid alone | sixteen parts | shares of 24, 32, 43: 8 KV heads, one 103 | 127 | 100, 100, 100; 4 heads
+//    77 | 115 | 73, 69, 67, two 103 | 127 | 99, 99, 100; 2 heads 86 | 114 | 58, 58, 60, two 78 | 115 | 73, 69, 67, three 89 | 121 | 85, 85, 83;
+//    one head 126 | 111 | 52, 52, 54.  Verify passes of 9 tokens, 4 heads 76 | 103 | 78, 78, 78; 2 heads 82 | 102 | 82, 79, 72.
+constexpr int kUnitCost = 4, kUnitCostWide = 8, kMinShare = 4, kMaxShare = 32, kMaxParts = 16, kWholeFree = 8;
 
 struct MetaM {  // one 64-byte record per ring stage, written by the producer
   int rows, tok0, flags, kvs;
@@ -818,25 +823,34 @@ __global__ void __launch_bounds__(threads_of(UMMA, UMMA ? 8 : MT * NS), (!UMMA &
   // share, 19.1 us against 19.6 us.  PARD verify, 128 units: 24.9 us against 34.0 us.)
   const int n_units = n_items * Hkv;
   const int per_cta = (n_units + (int)gridDim.x - 1) / (int)gridDim.x;  // whole units per CTA
+  auto cut = [&]() {
+    const int share = min(max(kMinShare, (misc[2] + UC + kMaxParts - 1) / kMaxParts), kMaxShare);
+    const long long most = MT == 1 || UMMA ? (T + share - 1) / share : T;
+    NC = T_real == 0 ? 1 : (long long)gridDim.x < most ? (int)gridDim.x : (int)most;
+    small = (T + 1) * (NC + 1) < (1LL << 31);
+    x0 = cta < NC ? range_begin(cta) : 0;
+    x1 = cta < NC ? range_begin(cta + 1) : 0;
+  };
   // p.whole_units: the caller asked for this form whatever the balance; such a launch never touches
   // the workspace.
+  // (Whole units have no use for the cut partition.  The form of 256 rows works it out first all the same: compiled in the other order
+  // its loops come out slower, a portion of 512 tokens behind 32768 310 us instead of 292.)
+  if constexpr (WIDE) cut();
   if (p.whole_units || (long long)per_cta * misc[2] * gridDim.x * 10 <= (long long)T_real * 13 + (MT == 1 ? (long long)gridDim.x * 10 * kWholeFree : 0)) {
     const int u0 = cta * per_cta, u1 = min(n_units, u0 + per_cta);
+    x0 = x1 = 0;
+    if constexpr (!WIDE) {
 #pragma unroll 1
-    for (int u = u0; u < u1; ++u) n_my += chunks_in(u / Hkv);
+      for (int u = u0; u < u1; ++u) n_my += chunks_in(u / Hkv);
+    }
     if (u0 < n_units) {
       const int it0 = u0 / Hkv, h0 = u0 - it0 * Hkv;
       x0 = (long long)prefix[it0] + (long long)h0 * ((prefix[it0 + 1] - prefix[it0]) / Hkv);
       const int it1 = (u1 - 1) / Hkv, h1 = (u1 - 1) - it1 * Hkv;
       x1 = (long long)prefix[it1] + (long long)(h1 + 1) * ((prefix[it1 + 1] - prefix[it1]) / Hkv);
     }
-  } else {
-    const int share = max(kMinShare, (misc[2] + UC + kMaxParts - 1) / kMaxParts);
-    const unsigned most = MT == 1 || UMMA ? ((unsigned)T + share - 1) / share : (unsigned)T;
-    NC = gridDim.x < most ? (int)gridDim.x : (int)most;
-    small = (T + 1) * (NC + 1) < (1LL << 31);
-    x0 = cta < NC ? range_begin(cta) : 0;
-    x1 = cta < NC ? range_begin(cta + 1) : 0;
+  } else if constexpr (!WIDE) {
+    cut();
     if (x1 > x0) n_my = UC ? chunks_between(x0, x1) : (int)(x1 - x0);
   }
 
@@ -856,6 +870,7 @@ __global__ void __launch_bounds__(threads_of(UMMA, UMMA ? 8 : MT * NS), (!UMMA &
     }
   }
   if (x1 <= x0) return;
+  if constexpr (WIDE) n_my = chunks_between(x0, x1);
   if (n_my <= 0) {
     gdc_wait();
     return;

@@ -50,3 +50,23 @@ def test_cut_units_of_many_query_rows(new, past):
     some = [b for b in range(B) if new[b]]
     for b, w in zip(some, _oracle(q[some], [ks[b] for b in some], [vs[b] for b in some], q_lens=[new[b] for b in some])):
         _check(got[b][:, : new[b]], w)
+
+
+@pytest.mark.parametrize("new", [1, 9])
+@pytest.mark.parametrize("heads,kv,lens", [(4, 1, [40000, 70]), (8, 2, [70001])])
+def test_long_units(heads, kv, lens, new):
+    """Units so long that a share's bound cuts them into more than sixteen parts."""
+    from pace_b200.llm.cache import KVCacheManager, KVCacheType
+    from pace_b200.ops import MultiHeadAttention
+    D, B = 128, len(lens)
+    g = torch.Generator().manual_seed(lens[0])
+    ks = [torch.randn(kv, n, D, generator=g).bfloat16().to(DEV) for n in lens]
+    vs = [torch.randn(kv, n, D, generator=g).bfloat16().to(DEV) for n in lens]
+    mgr = KVCacheManager(Cfg(2), max(lens) + 8, KVCacheType.BMC)
+    cached = [_fill(mgr, i, ks, vs) for i in range(2)]
+    q = torch.randn(2, B, heads, new, D, generator=g).bfloat16().to(DEV)
+    got = [MultiHeadAttention()(q[i], *cached[i]) for i in range(2)]
+    mgr.pool.check_status()
+    for i in range(2):
+        for b, w in enumerate(_oracle(q[i], ks, vs, q_lens=[new] * B)):
+            _check(got[i][b], w)
