@@ -520,14 +520,32 @@ Parts parts_of(const pace_step_t& st, int heads, int vdim, bool lightning) {
   p.total = p.add + p.tiles + p.kv + p.log_decay;
   return p;
 }
-// Prompts that are a chunk at most stay with the chunks of 64, which take one launch: 128 tokens 24.1 us (lightning) and 20.8 (state space)
-// against 24.7 and 26.8 here; 200 tokens 42.0 and 31.6 against 24.9 and 26.9.
-constexpr int kFewTokens = kChunk + 1;
 
 }  // namespace
 
+// Which of the two forms a step takes.  The chunks of 64 are one launch in which every sequence walks its chunks one after another (a
+// block per SM), the chunks of 128 three launches over all chunks side by side (two blocks per SM), whose last chunks are half empty.
+// Both are estimated, in us on the device, from what they showed over steps of 130 to 1024 tokens, 1 to 16 sequences and 16 to 64 heads
+// (state space of 64 / 128 values, lightning of 128), and with them a call: two launches and an allocation more cost the host 10 us
+// where nothing else is in flight.  Calls of the chunks of 64 and of 128, us: state space, 32 heads of 64, one prompt of 300 tokens 43.1 and
+// 49.2, of 400 53.7 and 50.1; 4 of 300 45.3 and 57.1, 8 of 500 117 and 113, 16 of 200 118 and 109; of 128 values, 4 of 600 106 and 121, one
+// of 300 56.0 and 50.9; lightning, 32 heads, one of 130 34.8 and 30.9, 4 of 300 54.1 and 64.2, 8 of 500 160 and 143.
+bool chunk_umma_pays(const pace_step_t& st, int heads, int vdim, bool lightning, int segments) {
+  if (st.max_count < kChunk + 1 || st.n_entries < 1) return false;
+  if (segments > 1) return true;        // (long sequences that leave SMs idle: the chunks of 64 go through twice)
+  const int vp = vdim <= 64 ? 64 : 128, n = st.n_entries, wide = vp / 64 - 1;
+  const float items = (float)heads * ((vdim + vp - 1) / vp);
+  const int waves = (int)((n * items + 147.f) / 148.f);
+  const float longest = (float)((st.max_count + 63) / 64), mean = fminf(longest, ceilf((float)st.n_tokens / (64.f * n)));
+  const float walk = waves <= 1 ? longest : fmaxf(longest, mean * waves + 0.5f * (longest - mean));
+  const float old_us = 3.5f + (wide ? 8.2f : 5.6f) * (lightning ? 1.11f : 1.f) * walk;
+  const float places = fminf((float)(st.n_tokens / kChunk + n), (float)n * ((st.max_count + kChunk - 1) / kChunk));
+  const float new_us = fmaxf(wide ? 24.f : 18.f, 8.f + (wide ? 0.126f : 0.073f) * places * items);
+  return lightning ? fmaxf(30.f, new_us + 9.f) < fmaxf(30.f, old_us + 4.5f) : fmaxf(50.f, new_us + 21.f) < fmaxf(40.f, old_us + 15.f);
+}
+
 uint64_t chunk_umma_bytes(const pace_step_t& st, int heads, int dim, int vdim, bool lightning) {
-  if (dim <= 64 || dim > 128 || dim % 8 || vdim % 8 || heads > 65535 || st.n_entries > 65535 || st.max_count < kFewTokens) return 0;
+  if (dim <= 64 || dim > 128 || dim % 8 || vdim % 8 || heads > 65535 || st.n_entries > 65535 || st.max_count < kChunk + 1) return 0;
   const Parts p = parts_of(st, heads, vdim, lightning);
   if (p.per_round > 65535 || (int64_t)heads * p.v_blocks > 65535) return 0;
   return p.total <= kBudget + 256 ? p.total : 0;

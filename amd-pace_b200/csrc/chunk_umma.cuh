@@ -24,7 +24,9 @@ struct ChunkArgs {
   unsigned char *tiles, *kv;
 };
 
-// Scratch of a step, 0 where the chunks of 64 are to be taken.
+// Whether the chunks of 128 are the faster form of a step (segments: into how many the chunks of 64 would cut a sequence).
+bool chunk_umma_pays(const pace_step_t& st, int heads, int vdim, bool lightning, int segments);
+// Scratch of a step, 0 where they cannot be taken.
 uint64_t chunk_umma_bytes(const pace_step_t& st, int heads, int dim, int vdim, bool lightning);
 // False: not for these operands or this much scratch (the chunks of 64 take them).
 bool chunk_umma_fits(const pace_step_t& st, const ChunkArgs& a, const void* workspace, uint64_t workspace_bytes);

@@ -384,7 +384,10 @@ int lightning_chunked(const pace_step_t& st, const pace_lightning_args_t& a, cud
 
 extern "C" uint64_t pace_lightning_scratch_bytes(const pace_step_t* st, int32_t heads, int32_t dim, int32_t vdim, int32_t dtype) {
   if (!st || st->max_count <= 1 || heads <= 0 || dim <= 0 || vdim <= 0 || dtype != PACE_DTYPE_BF16) return 0;
-  const uint64_t n = pace::chunk_umma_bytes(*st, heads, dim, vdim, true), old = pace_lightning_workspace_bytes(st->n_entries, st->max_count, heads, dim, vdim);
+  const uint64_t old = pace_lightning_workspace_bytes(st->n_entries, st->max_count, heads, dim, vdim);
+  const int segments = st->n_entries > 0 ? pace::plan_segments(st->n_entries, st->max_count, heads, vdim).segments : 1;
+  if (!pace::chunk_umma_pays(*st, heads, vdim, true, segments)) return old;
+  const uint64_t n = pace::chunk_umma_bytes(*st, heads, dim, vdim, true);
   return n > old ? n : old;
 }
 

@@ -415,7 +415,10 @@ int ssd_chunked(const pace_step_t& st, const pace_ssd_args_t& a, cudaStream_t s)
 
 extern "C" uint64_t pace_ssd_scratch_bytes(const pace_step_t* st, int32_t heads, int32_t state, int32_t vdim, int32_t dtype) {
   if (!st || st->max_count <= 1 || heads <= 0 || state <= 0 || vdim <= 0 || dtype != PACE_DTYPE_BF16) return 0;
-  const uint64_t n = pace::chunk_umma_bytes(*st, heads, state, vdim, false), old = pace_ssd_workspace_bytes(st->n_entries, st->max_count, heads, state, vdim);
+  const uint64_t old = pace_ssd_workspace_bytes(st->n_entries, st->max_count, heads, state, vdim);
+  const int segments = st->n_entries > 0 ? pace::plan_segments(st->n_entries, st->max_count, heads, vdim).segments : 1;
+  if (!pace::chunk_umma_pays(*st, heads, vdim, false, segments)) return old;
+  const uint64_t n = pace::chunk_umma_bytes(*st, heads, state, vdim, false);
   return n > old ? n : old;
 }
 

@@ -15,7 +15,7 @@ schema can say what an op writes.
 """
 import ctypes as C
 import math
-from typing import Optional
+from typing import Callable, Optional
 
 import torch
 
@@ -444,17 +444,17 @@ def _kv_append_conv(pool, pages, layer, step, qkv, taps, ring, q_norm, k_norm, c
         _C.check(_C.lib.pace_kv_append_conv(_pool(pool), layer, _step(step), C.byref(a), _stream(pages)), "pace_kv_append_conv")
 
 
-def _workspace(a, nbytes: int, device, fewer: Optional[int] = None) -> Optional[torch.Tensor]:
-    """Scratch of one launch (stream ordered: the allocator hands it out again only behind it); ``fewer`` bytes, with which
+def _workspace(a, nbytes: int, device, fewer: Optional[Callable[[], int]] = None) -> Optional[torch.Tensor]:
+    """Scratch of one launch (stream ordered: the allocator hands it out again only behind it); ``fewer()`` bytes, with which
     the launch takes another form, where the device has no room for ``nbytes``."""
     if not nbytes:
         return None
     try:
         ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
     except torch.OutOfMemoryError:
-        if fewer is None or fewer >= nbytes:
+        if fewer is None or fewer() >= nbytes:
             raise
-        return _workspace(a, fewer, device)
+        return _workspace(a, fewer(), device)
     a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
     return ws
 
@@ -476,7 +476,7 @@ def _ssd(entry: str):
             ws = None
             if taps is None and a.dtype == _C.DTYPE_BF16:
                 ws = _workspace(a, _C.lib.pace_ssd_scratch_bytes(_step(step), a.heads, a.state, a.vdim, a.dtype), out.device,
-                                _C.lib.pace_ssd_workspace_bytes(st.n_entries, st.max_count, a.heads, a.state, a.vdim))
+                                lambda: _C.lib.pace_ssd_workspace_bytes(st.n_entries, st.max_count, a.heads, a.state, a.vdim))
             _C.check(fn(_step(step), C.byref(a), _stream(out)), entry)
             del ws
     return impl
@@ -643,7 +643,7 @@ def _lightning(entry: str):
             ws = None
             if st.max_count > 1:
                 ws = _workspace(a, _C.lib.pace_lightning_scratch_bytes(_step(step), a.heads, a.dim, a.vdim, a.dtype), out.device,
-                                _C.lib.pace_lightning_workspace_bytes(st.n_entries, st.max_count, a.heads, a.dim, a.vdim))
+                                lambda: _C.lib.pace_lightning_workspace_bytes(st.n_entries, st.max_count, a.heads, a.dim, a.vdim))
             _C.check(fn(_step(step), C.byref(a), _stream(out)), entry)
             del ws
     return impl

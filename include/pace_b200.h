@@ -770,8 +770,8 @@ typedef struct {
 } pace_lightning_args_t;
 /* Scratch of a prefill (0: none).  Long sequences are cut into segments that run side by side. */
 uint64_t pace_lightning_workspace_bytes(int32_t n_entries, int32_t max_count, int32_t heads, int32_t dim, int32_t vdim);
-/* The same for one step, with what chunks of 128 tokens on tcgen05 take where the step has enough of them: 512 MB at most, beyond which
- * a step goes through in rounds (at least the figure above; with less the chunks of 64 are taken). */
+/* The same for one step, with what chunks of 128 tokens on tcgen05 take where they are the faster form of it: 512 MB at most, beyond
+ * which a step goes through in rounds (at least the figure above; with less the chunks of 64 are taken). */
 uint64_t pace_lightning_scratch_bytes(const pace_step_t* step, int32_t heads, int32_t dim, int32_t vdim, int32_t dtype);
 int pace_lightning_prefill(const pace_step_t* step, const pace_lightning_args_t* a, void* stream);
 int pace_lightning_step(const pace_step_t* step, const pace_lightning_args_t* a, void* stream);
