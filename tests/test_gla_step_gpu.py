@@ -1,5 +1,5 @@
-"""One token per sequence of gated linear attention: few heads (whole heads in registers) and many (rows in passes), odd sizes, fresh
-sequences, against 64-bit arithmetic."""
+"""One token per sequence of gated linear attention: few heads and more than the SMs hold at once, odd sizes, fresh sequences, against
+64-bit arithmetic."""
 from types import SimpleNamespace
 
 import pytest
